@@ -128,6 +128,15 @@ int slayer_b200_loihi_get_spikes_delayed(float *delayed, float *v, float *u, con
                                          uint32_t vDecay, uint32_t refDelay, int64_t delay, void *stream);
 
 /*
+ * slayer_b200_loihi_get_spikes_delayed for callers that keep neither voltage nor current (a layer
+ * through which no gradient flows): 8 bytes per element.  The same spikes as getSpikes<float>()
+ * (src/cuda/spikeLoihiKernels.h:75-96), delayed; the same limits.
+ */
+int slayer_b200_loihi_spikes_only(float *delayed, const float *w, int64_t rows, int64_t T,
+                                  uint32_t wgtExp, uint32_t theta, uint32_t iDecay,
+                                  uint32_t vDecay, uint32_t refDelay, int64_t delay, void *stream);
+
+/*
  * Surrogate gradient of the spike function, fused into one pass:
  *   out[i] = g[i] * ( scale / tau * exp(-|u[i] - theta| / tau) ),   i < n.
  * `out` may alias `g`.  Replaces the chain of elementwise tensor operations in

@@ -182,7 +182,7 @@ struct LoihiRow {
 // Two wide tiles of the same rows and steps to two arrays of the same shape: the row, its skew,
 // the bounds and the offset are worked out once per pass and shared by the two stores; the
 // spike samples of the same tile are expanded from bit masks in the same pass.
-template <bool SKEW, bool WRITE_U>
+template <bool SKEW, bool WRITE_U, bool WRITE_V>
 __device__ __forceinline__ void wide_store_loihi(const float *tile_u, const float *tile_v, const unsigned *masks,
                                                  float *gu, float *gv, float *gs, int64_t row0, int64_t rows,
                                                  int j, int T, int lane, int skew0)
@@ -201,13 +201,13 @@ __device__ __forceinline__ void wide_store_loihi(const float *tile_u, const floa
         if (t >= T || t + 4 <= 0) continue;
         const int wd = hoff + tile_word(r, c);
         const float4 vu = WRITE_U ? *reinterpret_cast<const float4 *>(tile_u + wd) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        const float4 vv = *reinterpret_cast<const float4 *>(tile_v + wd);
+        const float4 vv = WRITE_V ? *reinterpret_cast<const float4 *>(tile_v + wd) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         const unsigned m = mhalf[r] >> c;
         const float4 vs = make_float4((m & 1u) ? 1.0f : 0.0f, (m & 2u) ? 1.0f : 0.0f, (m & 4u) ? 1.0f : 0.0f, (m & 8u) ? 1.0f : 0.0f);
         const int64_t off = (row0 + r) * (int64_t)T + t;
         if (t >= 0 && t + 4 <= T) {
             if (WRITE_U) *reinterpret_cast<float4 *>(gu + off) = vu;
-            *reinterpret_cast<float4 *>(gv + off) = vv;
+            if (WRITE_V) *reinterpret_cast<float4 *>(gv + off) = vv;
             *reinterpret_cast<float4 *>(gs + off) = vs;
         } else {
             const float eu[4] = {vu.x, vu.y, vu.z, vu.w};
@@ -217,7 +217,7 @@ __device__ __forceinline__ void wide_store_loihi(const float *tile_u, const floa
             for (int k = 0; k < 4; ++k)
                 if (t + k >= 0 && t + k < T) {
                     if (WRITE_U) gu[off + k] = eu[k];
-                    gv[off + k] = ev[k];
+                    if (WRITE_V) gv[off + k] = ev[k];
                     gs[off + k] = es[k];
                 }
         }
@@ -235,12 +235,13 @@ __device__ __forceinline__ void wide_store_loihi(const float *tile_u, const floa
 // what the definition prescribes for t = 0 (0 > theta cannot fire because theta >= 0 here).
 //
 // WRITE_U = false leaves the current out (callers that only keep spikes and voltage: 12 instead
-// of 16 bytes per element).  `delay` (0 .. 63 steps) writes the spikes already delayed,
+// of 16 bytes per element), WRITE_V = false the voltage too (no gradient: 8 bytes, and without the
+// voltage tile 13 warps instead of 8 per SM).  131072 x 1450, spikes then shift, no gradient: 1143 -> 781 us.  `delay` (0 .. 63 steps) writes the spikes already delayed,
 // s_out[t] = s[t - delay]: a Loihi layer is always followed by a delay of one step, and the
 // spike bits of a tile only need a 64-bit shift with carry from the previous tile for that, so
 // the separate shift pass (8 bytes per element) disappears.
 // ---------------------------------------------------------------------------------------
-template <bool SKEW, bool WRITE_U>
+template <bool SKEW, bool WRITE_U, bool WRITE_V>
 __global__ void __launch_bounds__(256)
 loihi_get_spikes_wide_kernel(float *s, float *v, float *u, const float *w,
                              int64_t rows, int T, unsigned weightScale, int theta,
@@ -250,9 +251,9 @@ loihi_get_spikes_wide_kernel(float *s, float *v, float *u, const float *w,
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int warps_per_block = blockDim.x >> 5;
-    float *tiles = smem + warp * ((depth + 1) * kWideWords + 2 * kTile);
+    float *tiles = smem + warp * ((depth + (WRITE_V ? 1 : 0)) * kWideWords + 2 * kTile);
     float *tile_v = tiles + depth * kWideWords;
-    unsigned *masks = reinterpret_cast<unsigned *>(tile_v + kWideWords);
+    unsigned *masks = reinterpret_cast<unsigned *>(tile_v + (WRITE_V ? kWideWords : 0));
     const float vMarkF = (float)vDecayMark;
 
     const int ntiles = SKEW ? skew_wide_tiles(T) : (T + kWide - 1) / kWide;
@@ -318,7 +319,7 @@ loihi_get_spikes_wide_kernel(float *s, float *v, float *u, const float *w,
                 for (int k = 0; k < 4; ++k)
                     if (st.step(wv[k], weightScale, theta, iKeep, vKeep, vMarkF, refDelay, uo[k], vo[k])) mh |= 1u << (c4 * 4 + k);
                 if (WRITE_U) *reinterpret_cast<float4 *>(th + tile_chunk(lane, c4)) = make_float4(uo[0], uo[1], uo[2], uo[3]);
-                *reinterpret_cast<float4 *>(tv + tile_chunk(lane, c4)) = make_float4(vo[0], vo[1], vo[2], vo[3]);
+                if (WRITE_V) *reinterpret_cast<float4 *>(tv + tile_chunk(lane, c4)) = make_float4(vo[0], vo[1], vo[2], vo[3]);
                 cur = nxt;
             }
             if (h == 0) m[0] = mh;
@@ -335,7 +336,7 @@ loihi_get_spikes_wide_kernel(float *s, float *v, float *u, const float *w,
         }
         __syncwarp();
 
-        wide_store_loihi<SKEW, WRITE_U>(tile, tile_v, masks, u, v, s, row0, rows, it, T, lane, skew);
+        wide_store_loihi<SKEW, WRITE_U, WRITE_V>(tile, tile_v, masks, u, v, s, row0, rows, it, T, lane, skew);
         __syncwarp();
         if (++it == ntiles) {
             it = 0;
@@ -373,21 +374,24 @@ static int launch_loihi(const LoihiArgs &a)
     return check_launch("loihi_get_spikes kernel launch");
 }
 
+// a.u and a.v may be null: that output is not wanted
 static int launch_loihi_wide(const LoihiArgs &a, int delay = 0)
 {
     const int64_t nblocks = ceil_div(a.rows, kTile);
     // prefetch depth 4 when every warp of the launch is resident at once even with the larger
     // footprint (then latency, not bandwidth, bounds the launch), depth 2 otherwise
-    const size_t deep_bytes = (5 * kWideWords + 2 * kTile) * sizeof(float);
+    const int vtiles = a.v ? 1 : 0;
+    const size_t deep_bytes = ((4 + vtiles) * kWideWords + 2 * kTile) * sizeof(float);
     const int depth = nblocks <= (int64_t)((216 * 1024) / deep_bytes) * sm_count() ? 4 : 2;
-    const size_t warp_bytes = (size_t)((depth + 1) * kWideWords + 2 * kTile) * sizeof(float);
+    const size_t warp_bytes = (size_t)((depth + vtiles) * kWideWords + 2 * kTile) * sizeof(float);
     int warps, grid;
     spike_launch_shape(nblocks, warp_bytes, warps, grid);
     const size_t smem = (size_t)warps * warp_bytes;
     // rows that start on 32-byte boundaries need no skew
     const bool skew = (a.T & 7) != 0 || (reinterpret_cast<uintptr_t>(a.w) & 31u) != 0;
-    auto kern = a.u ? (skew ? loihi_get_spikes_wide_kernel<true, true> : loihi_get_spikes_wide_kernel<false, true>)
-                    : (skew ? loihi_get_spikes_wide_kernel<true, false> : loihi_get_spikes_wide_kernel<false, false>);
+    auto kern = a.u ? (skew ? loihi_get_spikes_wide_kernel<true, true, true> : loihi_get_spikes_wide_kernel<false, true, true>)
+              : a.v ? (skew ? loihi_get_spikes_wide_kernel<true, false, true> : loihi_get_spikes_wide_kernel<false, false, true>)
+                    : (skew ? loihi_get_spikes_wide_kernel<true, false, false> : loihi_get_spikes_wide_kernel<false, false, false>);
     int rc = reserve_dynamic_smem((const void *)kern, smem);
     if (rc) return rc;
     kern<<<(unsigned)grid, warps * 32, smem, a.stream>>>(a.s, a.v, a.u, a.w, a.rows, a.T, a.weightScale, a.theta,
@@ -424,6 +428,29 @@ extern "C" int slayer_b200_loihi_get_spikes(float *s, float *v, float *u, const 
         case 2: return launch_loihi<2>(a);
         default: return launch_loihi<1>(a);
     }
+}
+
+extern "C" int slayer_b200_loihi_spikes_only(float *delayed, const float *w, int64_t rows, int64_t T,
+                                             uint32_t wgtExp, uint32_t theta, uint32_t iDecay,
+                                             uint32_t vDecay, uint32_t refDelay, int64_t delay, void *stream_)
+{
+    using namespace sb200;
+    clear_error();
+    SB200_REQUIRE(rows >= 0 && T >= 0, "loihi_spikes_only: negative size");
+    SB200_REQUIRE(T < (1LL << 31) - 64, "loihi_spikes_only: T=%lld too large", (long long)T);
+    SB200_REQUIRE(refDelay >= 1, "loihi_spikes_only: refDelay must be >= 1");
+    SB200_REQUIRE(wgtExp <= 25, "loihi_spikes_only: wgtExp=%u out of range", wgtExp);
+    if (rows == 0 || T == 0) return SLAYER_B200_OK;
+    SB200_REQUIRE(delayed && w, "loihi_spikes_only: null pointer");
+    SB200_REQUIRE(delayed != w, "loihi_spikes_only: buffers must be distinct");
+    if (delay < 0 || delay > 63 || theta >= 0x80000000u || !all_aligned16({delayed, w})) {
+        set_error("loihi_spikes_only: needs a delay of 0 .. 63 steps, 16-byte aligned buffers and a threshold "
+                  "below 2^31; otherwise run slayer_b200_loihi_get_spikes and slayer_b200_shift_scalar");
+        return SLAYER_B200_EUNSUPPORTED;
+    }
+    const LoihiArgs a = {delayed, nullptr, nullptr, w, rows, (int)T, 1u << (6 + wgtExp), (int)theta,
+                         4096u - iDecay, 4096u - vDecay, (int)vDecay, refDelay, (cudaStream_t)stream_};
+    return launch_loihi_wide(a, (int)delay);
 }
 
 extern "C" int slayer_b200_loihi_get_spikes_delayed(float *delayed, float *v, float *u, const float *w,

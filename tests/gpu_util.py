@@ -159,3 +159,11 @@ def c_loihi_delayed(w, wgtExp, theta, iDecay, vDecay, refDelay, delay, current=T
     capi.call("slayer_b200_loihi_get_spikes_delayed", ptr(d), ptr(v), ptr(u) if current else None, ptr(w), rows, T,
               int(wgtExp), int(theta), int(iDecay), int(vDecay), int(refDelay), int(delay), stream())
     return d, v, u
+
+
+def c_loihi_spikes_only(w, wgtExp, theta, iDecay, vDecay, refDelay, delay):
+    d = torch.full_like(w, float("nan"))
+    rows, T = rows_T(w)
+    capi.call("slayer_b200_loihi_spikes_only", ptr(d), ptr(w), rows, T, int(wgtExp), int(theta), int(iDecay), int(vDecay),
+              int(refDelay), int(delay), stream())
+    return d

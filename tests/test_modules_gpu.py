@@ -362,3 +362,6 @@ def test_loihi_spike_delayed_layer_function_equals_the_two_steps():
         yb.backward(gout)
         assert torch.equal(ya, yb) and ya.sum() > 0
         assert torch.equal(a.grad, b.grad)
+        # no gradient wanted: the voltage is not kept
+        assert torch.equal(net.delayShift(net.spikeLoihi(w), float(steps), 1.0), ya)
+        assert torch.equal(net.spikeLoihiDelayed(w, steps), ya)

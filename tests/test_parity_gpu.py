@@ -476,7 +476,25 @@ def test_loihi_get_spikes_delayed_equals_get_spikes_then_shift(T, delay):
             np.testing.assert_array_equal(G.host(u), u_o)
     s, _, _ = G.c_loihi(wd, *params)
     np.testing.assert_array_equal(G.host(d), G.host(G.c_shift_scalar(s, delay, 1.0)))
+    np.testing.assert_array_equal(G.host(G.c_loihi_spikes_only(wd, *params, delay)), want_d)
     assert T < 30 or s_o.sum() > 0
+
+
+@pytest.mark.parametrize("off,T,delay,theta", [(0, 65, 0, 5120), (0, 65, 64, 5120), (1, 63, 0, 5120), (1, 129, 2, 5120),
+                                               (0, 130, 1, 0x80000000)])
+def test_loihi_spikes_only_operator_equals_the_full_one(off, T, delay, theta):
+    """Without the voltage, on the fused kernel and where the operator falls back: the same spikes."""
+    import slayerpytorch_b200
+    _, lc = slayerpytorch_b200.load_ops()
+    rng = np.random.RandomState(T + off)
+    n = 37 * T
+    w = (np.round((rng.rand(n + off) - 0.5) * 90) * (rng.rand(n + off) < 0.3)).astype(np.float32)
+    wd = G.dev(w)[off:].view(1, 37, 1, 1, T)
+    (got,) = lc.getSpikesDelayed(wd, 0, theta, 1024, 128, 1, delay, False, False)
+    want = co.shift(co.loihi_get_spikes(w[off:].reshape(37, T), 0, theta, 1024, 128, 1)[0], float(delay), 1.0)
+    np.testing.assert_array_equal(G.host(got).reshape(37, T), want)
+    with pytest.raises(RuntimeError):
+        lc.getSpikesDelayed(wd, 0, theta, 1024, 128, 1, delay, True, False)
 
 
 def test_loihi_get_spikes_delayed_sizes_outside_the_fused_path():
