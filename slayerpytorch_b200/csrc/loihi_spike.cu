@@ -151,10 +151,14 @@ loihi_get_spikes_kernel(float *s, float *v, float *u, const float *w,
 // One time step of the neuron for one row.  The decays are written on the magnitude with the
 // sign folded back in by xor / subtract (sm = 0 or -1): for every 32-bit state, INT_MIN
 // included, this is the reference's expression sgn(x) * ((sgn(x) * x * keep) >> 12) evaluated
-// modulo 2^32 with a logical shift.
+// modulo 2^32 with a logical shift.  A row's steps are a serial chain, and a scheduler has two or
+// three rows' chains to interleave, so what need not be on it is not: the magnitude is a maximum,
+// the subtraction of the sign is folded into the term that is added anyway, and the countdown is
+// kept as the next step will see it, so that a spike reaches the next step's comparison through
+// one select.
 struct LoihiRow {
     int uOld, vOld;
-    unsigned refLeft;           // steps until the refractory state clears (0 = not refractory)
+    unsigned refLeft;           // steps, the next one not counted, until the refractory state clears
 
     __device__ __forceinline__ void reset() { uOld = 0; vOld = 0; refLeft = 0; }
 
@@ -162,16 +166,15 @@ struct LoihiRow {
     __device__ __forceinline__ bool step(float wv, unsigned weightScale, int theta, unsigned iKeep, unsigned vKeep,
                                          float vMarkF, unsigned refDelay, float &uo, float &vo)
     {
-        const int us = uOld >> 31, vs = vOld >> 31;
-        const unsigned udec = (((unsigned)((uOld ^ us) - us) * iKeep) >> 12);
-        const unsigned vdec = (((unsigned)((vOld ^ vs) - vs) * vKeep) >> 12);
-        const unsigned uT = (unsigned)(((int)udec ^ us) - us) + weightScale * (unsigned)__float2int_rz(wv);
-        const int vT = (int)((unsigned)(((int)vdec ^ vs) - vs) + uT);
-        if (refLeft != 0) --refLeft;
+        const unsigned us = (unsigned)(uOld >> 31), vs = (unsigned)(vOld >> 31);
+        const unsigned umag = (unsigned)max(uOld, (int)(0u - (unsigned)uOld));
+        const unsigned vmag = (unsigned)max(vOld, (int)(0u - (unsigned)vOld));
+        const unsigned uT = (((umag * iKeep) >> 12) ^ us) + (weightScale * (unsigned)__float2int_rz(wv) - us);
+        const int vT = (int)((((vmag * vKeep) >> 12) ^ vs) + (uT - vs));
         const bool quiet = refLeft == 0;
         const bool spk = (vT > theta) && quiet;
         vOld = (quiet && !spk) ? vT : 0;
-        if (spk) refLeft = refDelay;
+        refLeft = spk ? refDelay - 1u : refLeft - (quiet ? 0u : 1u);
         uOld = (int)uT;
         uo = (float)uOld;
         vo = spk ? vMarkF : (float)vOld;
@@ -184,7 +187,7 @@ struct LoihiRow {
 // spike samples of the same tile are expanded from bit masks in the same pass.
 template <bool SKEW, bool WRITE_U, bool WRITE_V>
 __device__ __forceinline__ void wide_store_loihi(const float *tile_u, const float *tile_v, const unsigned *masks,
-                                                 float *gu, float *gv, float *gs, int64_t row0, int64_t rows,
+                                                 float *__restrict__ gu, float *__restrict__ gv, float *__restrict__ gs, int64_t row0, int64_t rows,
                                                  int j, int T, int lane, int skew0)
 {
     const int c16 = lane & 15;
@@ -193,6 +196,21 @@ __device__ __forceinline__ void wide_store_loihi(const float *tile_u, const floa
     const unsigned *mhalf = masks + (c16 >> 3) * kTile;
     const int c = (c16 & 7) * 4;
     const int64_t nrow = rows - row0;
+    if (wide_inner<SKEW>(row0, rows, j, T)) {
+        int64_t at = (row0 + rsub) * (int64_t)T + (kWide * j + c16 * 4);
+#pragma unroll
+        for (int i = 0; i < kTile / 2; ++i, at += 2 * (int64_t)T) {
+            const int r = i * 2 + rsub;
+            const int wd = hoff + tile_word(r, c);
+            const int64_t off = at - (SKEW ? row_skew(skew0, r, T) : 0);
+            const unsigned m = mhalf[r] >> c;
+            if (WRITE_U) *reinterpret_cast<float4 *>(gu + off) = *reinterpret_cast<const float4 *>(tile_u + wd);
+            if (WRITE_V) *reinterpret_cast<float4 *>(gv + off) = *reinterpret_cast<const float4 *>(tile_v + wd);
+            *reinterpret_cast<float4 *>(gs + off) =
+                make_float4((m & 1u) ? 1.0f : 0.0f, (m & 2u) ? 1.0f : 0.0f, (m & 4u) ? 1.0f : 0.0f, (m & 8u) ? 1.0f : 0.0f);
+        }
+        return;
+    }
 #pragma unroll
     for (int i = 0; i < kTile / 2; ++i) {
         const int r = i * 2 + rsub;

@@ -338,6 +338,7 @@ srm_get_spikes_wide_kernel(float *s, float *u, const float *__restrict__ nu,
     int skew_next = skew;                                  // of the block being prefetched
     unsigned q = 0;                 // tiles walked so far: buffer = q & (depth - 1)
     const unsigned dmask = (unsigned)depth - 1u;
+    unsigned long long prev_bits = 0ull;                   // spike bits of the previous tile of this lane's row
 
     auto prefetch = [&](float *dst) {
         wide_prefetch_skew<SKEW>(dst, u, rb_next * kTile, rows, it_next, T, lane, skew_next, -INFINITY);
@@ -358,6 +359,7 @@ srm_get_spikes_wide_kernel(float *s, float *u, const float *__restrict__ nu,
         if (it == 0) {
             st.reset();
             ring_reset(ring);
+            prev_bits = 0ull;
         }
         if (rb_next < nblocks) prefetch(tiles + ((q + dmask) & dmask) * kWideWords);
         cp_async_commit();
@@ -381,7 +383,13 @@ srm_get_spikes_wide_kernel(float *s, float *u, const float *__restrict__ nu,
         masks[kTile + lane] = m1;
         __syncwarp();
 
-        wide_store_skew<SKEW>(tile, u, row0, rows, it, T, lane, skew);
+        // rows that neither a spike of this tile nor one of the nuEff - 1 steps before it can have
+        // changed are not written back (as in the kernel below)
+        const unsigned long long cur_bits = ((unsigned long long)m1 << 32) | m0;
+        const int reach = nuEff - 1;
+        const bool row_changed = cur_bits != 0ull || reach > kWide || (reach > 0 && (prev_bits >> (kWide - reach)) != 0ull);
+        prev_bits = cur_bits;
+        wide_store_skew<SKEW>(tile, u, row0, rows, it, T, lane, skew, __ballot_sync(0xffffffffu, row_changed));
         wide_store_spikes_skew<SKEW>(masks, s, row0, rows, it, T, lane, skew, spikeVal);
         __syncwarp();
         if (++it == ntiles) {

@@ -237,6 +237,17 @@ constexpr int kWideWords = 2 * kTileWords;
 // number of wide tiles that cover a row of T samples for every skew (0..7)
 __host__ __device__ inline int skew_wide_tiles(int T) { return (T + 7 + kWide - 1) / kWide; }
 
+// true (for the whole warp) if every sample of the wide tile exists: then its fill and its drain
+// are straight runs of 16-byte accesses.  A warp's fill and drain are in series with its walk, and
+// only 8 to 13 warps fit an SM, so their length counts: with the bounds tested per access, a branch
+// each, a warp's accesses went out one at a time.  (Loihi 131072 x 1450, spikes only 460 -> 381 us;
+// 1048576 x 1450 with the voltage 4.49 -> 4.08 ms; SRM 191664 x 301 237 -> 217 us.)
+template <bool SKEW>
+__device__ __forceinline__ bool wide_inner(int64_t row0, int64_t rows, int j, int T)
+{
+    return row0 + kTile <= rows && kWide * j >= (SKEW ? 7 : 0) && kWide * j + kWide <= T;
+}
+
 template <bool SKEW = true>
 __device__ __forceinline__ void wide_prefetch_skew(float *tile, const float *g, int64_t row0, int64_t rows,
                                                    int j, int T, int lane, int skew0, float pad)
@@ -246,6 +257,15 @@ __device__ __forceinline__ void wide_prefetch_skew(float *tile, const float *g, 
     float *half = tile + (c16 >> 3) * kTileWords;
     const int c = (c16 & 7) * 4;                // column inside the half
     const int64_t nrow = rows - row0;
+    if (wide_inner<SKEW>(row0, rows, j, T)) {
+        const float *src = g + (row0 + rsub) * (int64_t)T + (kWide * j + c16 * 4);
+#pragma unroll
+        for (int i = 0; i < kTile / 2; ++i, src += 2 * (int64_t)T) {
+            const int r = i * 2 + rsub;
+            cp_async<16>(half + tile_word(r, c), src - (SKEW ? row_skew(skew0, r, T) : 0), true);
+        }
+        return;
+    }
 #pragma unroll
     for (int i = 0; i < kTile / 2; ++i) {
         const int r = i * 2 + rsub;
@@ -282,19 +302,30 @@ __device__ __forceinline__ void store_clipped4(float *row, int t, int T, const f
     }
 }
 
+// Rows whose bit in `changed` is not set are left as they are in global memory.
 template <bool SKEW = true>
 __device__ __forceinline__ void wide_store_skew(const float *tile, float *g, int64_t row0, int64_t rows,
-                                                int j, int T, int lane, int skew0)
+                                                int j, int T, int lane, int skew0, unsigned changed)
 {
     const int c16 = lane & 15;
     const int rsub = lane >> 4;
     const float *half = tile + (c16 >> 3) * kTileWords;
     const int c = (c16 & 7) * 4;
     const int64_t nrow = rows - row0;
+    if (wide_inner<SKEW>(row0, rows, j, T)) {
+        float *dst = g + (row0 + rsub) * (int64_t)T + (kWide * j + c16 * 4);
+#pragma unroll
+        for (int i = 0; i < kTile / 2; ++i, dst += 2 * (int64_t)T) {
+            const int r = i * 2 + rsub;
+            const float4 v = *reinterpret_cast<const float4 *>(half + tile_word(r, c));
+            if (changed >> r & 1u) *reinterpret_cast<float4 *>(dst - (SKEW ? row_skew(skew0, r, T) : 0)) = v;
+        }
+        return;
+    }
 #pragma unroll
     for (int i = 0; i < kTile / 2; ++i) {
         const int r = i * 2 + rsub;
-        if (r >= nrow) continue;
+        if (r >= nrow || !(changed >> r & 1u)) continue;
         const int t = kWide * j - (SKEW ? row_skew(skew0, r, T) : 0) + c16 * 4;
         store_clipped4(g + (row0 + r) * (int64_t)T, t, T, *reinterpret_cast<const float4 *>(half + tile_word(r, c)));
     }
@@ -311,6 +342,17 @@ __device__ __forceinline__ void wide_store_spikes_skew(const unsigned *masks, fl
     const unsigned *half = masks + (c16 >> 3) * kTile;
     const int sh = (c16 & 7) * 4;
     const int64_t nrow = rows - row0;
+    if (wide_inner<SKEW>(row0, rows, j, T)) {
+        float *dst = g + (row0 + rsub) * (int64_t)T + (kWide * j + c16 * 4);
+#pragma unroll
+        for (int i = 0; i < kTile / 2; ++i, dst += 2 * (int64_t)T) {
+            const int r = i * 2 + rsub;
+            const unsigned m = half[r] >> sh;
+            *reinterpret_cast<float4 *>(dst - (SKEW ? row_skew(skew0, r, T) : 0)) =
+                make_float4((m & 1u) ? value : 0.0f, (m & 2u) ? value : 0.0f, (m & 4u) ? value : 0.0f, (m & 8u) ? value : 0.0f);
+        }
+        return;
+    }
 #pragma unroll
     for (int i = 0; i < kTile / 2; ++i) {
         const int r = i * 2 + rsub;
