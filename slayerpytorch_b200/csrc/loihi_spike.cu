@@ -254,7 +254,8 @@ __device__ __forceinline__ void wide_store_loihi(const float *tile_u, const floa
 //
 // WRITE_U = false leaves the current out (callers that only keep spikes and voltage: 12 instead
 // of 16 bytes per element), WRITE_V = false the voltage too (no gradient: 8 bytes, and without the
-// voltage tile 13 warps instead of 8 per SM).  131072 x 1450, spikes then shift, no gradient: 1143 -> 781 us.  `delay` (0 .. 63 steps) writes the spikes already delayed,
+// voltage tile 13 warps instead of 8 per SM).  131072 x 1450, spikes then shift, no gradient:
+// 1143 -> 781 us.  `delay` (0 .. 63 steps) writes the spikes already delayed,
 // s_out[t] = s[t - delay]: a Loihi layer is always followed by a delay of one step, and the
 // spike bits of a tile only need a 64-bit shift with carry from the previous tile for that, so
 // the separate shift pass (8 bytes per element) disappears.
