@@ -14,6 +14,7 @@ to the new binaries, which is all the reference's own ``slayer.py`` / ``slayerLo
 to run on them unchanged.  There is no CPU fallback: if the binaries are missing, importing
 the operators fails.
 """
+import importlib
 import os
 import sys
 
@@ -38,6 +39,9 @@ def load_ops():
     """Import and return ``(slayerCuda, slayerLoihiCuda)``; raises if they are not built or
     if the names resolve to some other implementation."""
     install()
+    # if lib/ did not exist yet when the package was imported (a clean checkout building itself), the
+    # import system has noted that this path entry holds nothing
+    importlib.invalidate_caches()
     import torch  # noqa: F401  (the extension modules link against libtorch)
     try:
         import slayerCuda

@@ -1,4 +1,9 @@
 """CPU: host-side logic of the package (kernel construction, module loading)."""
+import os
+import shutil
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -11,6 +16,26 @@ def test_extension_modules_import_and_identify_themselves():
     for name in ("getSpikes", "conv", "corr", "shift", "spikeGrad"):
         assert hasattr(sc, name)
     assert hasattr(lc, "getSpikes")
+
+
+def test_operators_built_after_the_package_was_imported_are_found(tmp_path):
+    """A clean checkout imports the package, builds lib/ and loads the operators in one process."""
+    package = tmp_path / "slayerpytorch_b200"
+    package.mkdir()
+    shutil.copy(slayerpytorch_b200.__file__, package)
+    script = """
+import os
+import slayerpytorch_b200 as package
+import wave                                 # any import: the path entry is looked at, and is no folder yet
+os.mkdir(package.LIB_DIR)
+for name in ("slayerCuda", "slayerLoihiCuda"):
+    with open(os.path.join(package.LIB_DIR, name + ".py"), "w") as f:
+        f.write("backend = 'slayer_b200'")
+assert [m.__name__ for m in package.load_ops()] == ["slayerCuda", "slayerLoihiCuda"]
+"""
+    env = dict(os.environ, PYTHONPATH=str(tmp_path))
+    done = subprocess.run([sys.executable, "-c", script], env=env, cwd=tmp_path, capture_output=True, text=True)
+    assert done.returncode == 0, done.stderr
 
 
 def test_operators_refuse_cpu_tensors():
