@@ -132,7 +132,9 @@ extern "C" int slayer_b200_num_spikes_loss(float *grad, double *row_sq, const fl
     SB200_REQUIRE(grad && row_sq && s && desired_count && (filter || K == 0), "num_spikes_loss: null pointer");
     SB200_REQUIRE(grad != s, "num_spikes_loss: grad must not alias s");
     const int64_t Keff = K < T ? K : T;
-    if (T >= (1 << 24) || sizeof(float) * ((size_t)Keff + 8 * (size_t)T) > 200 * 1024) {      // (the kernel takes less)
+    // taps and zeros, the row, the error signal and zeros
+    const size_t smem = T < (1 << 24) ? sizeof(float) * (3 * (size_t)Keff + 2 * (size_t)loss_span((int)T)) : SIZE_MAX;
+    if (smem > 200 * 1024) {
         set_error("num_spikes_loss: rows of %lld steps do not fit the kernel's shared memory", (long long)T);
         return SLAYER_B200_EUNSUPPORTED;
     }
@@ -140,8 +142,6 @@ extern "C" int slayer_b200_num_spikes_loss(float *grad, double *row_sq, const fl
     int64_t lo = start < 0 ? start + T : start, hi = stop < 0 ? stop + T : stop;
     lo = lo < 0 ? 0 : (lo > T ? T : lo);
     hi = hi < 0 ? 0 : (hi > T ? T : hi);
-    // taps and zeros, the row, the error signal and zeros
-    const size_t smem = sizeof(float) * (3 * (size_t)Keff + 2 * (size_t)loss_span((int)T));
     int rc = reserve_dynamic_smem((const void *)num_spikes_loss_kernel, smem);
     if (rc) return rc;
     int64_t blocks = rows;

@@ -66,7 +66,8 @@ class spikeLoss(torch.nn.Module):
         lo, hi = slice(start, stop).indices(T)[:2]        # the slice the reference takes, made explicit
 
         if spikeOut.is_cuda and spikeOut.dtype == torch.float32 and self.fused and stop != start and T <= 8192:
-            # one kernel for the loss and its gradient (same arithmetic as the expressions below)
+            # one kernel for the loss and its gradient (same arithmetic as the expressions below); rows of up to
+            # 8192 steps fit its shared memory with any filter (2 words per step, and 3 per tap, of which T count)
             onehot = desiredClass.to(spikeOut.device)
             desired = torch.where(onehot == True, float(count[True]), float(count[False]))    # noqa: E712
             desired = desired.to(torch.float32).expand(spikeOut.shape[:-1] + (1,)).reshape(-1).contiguous()

@@ -59,6 +59,10 @@ def test_argument_validation_needs_no_gpu():
     # Loihi refractory delay of zero is undefined in the reference and rejected here
     assert lib.slayer_b200_loihi_get_spikes(one, one, one, one, 2, 4, 0, 80, 1, 1, 0, null) == -1
     assert b"refDelay" in lib.slayer_b200_last_error()
+    # rows that do not fit the loss kernel's shared memory are refused, however long
+    for T in (25600, 1 << 31):
+        assert lib.slayer_b200_num_spikes_loss(one, one, ctypes.c_void_p(32), one, one, 2, T, 77, 0, T, 1.0, 1.0, null) == -3
+        assert b"shared memory" in lib.slayer_b200_last_error()
     # empty work is a successful no-op
     assert lib.slayer_b200_conv(null, null, null, 0, 4, 2, 1.0, null) == 0
     assert lib.slayer_b200_shift_lut(null, null, null, 0, 5, 4, 1.0, null) == 0

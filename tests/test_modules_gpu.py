@@ -314,7 +314,8 @@ def test_num_spikes_loss_against_a_host_restatement():
 
 
 @pytest.mark.parametrize("Ts,region,shape", [(1.0, (0, 300), (64, 10, 1, 1, 300)), (1.0, (40, 260), (5, 10, 1, 1, 300)),
-                                             (0.5, (10, 120), (3, 4, 2, 2, 300)), (1.0, (0, 2000), (2, 7, 1, 1, 2000))])
+                                             (0.5, (10, 120), (3, 4, 2, 2, 300)), (1.0, (0, 2000), (2, 7, 1, 1, 2000)),
+                                             (1.0, (0, 6400), (2, 3, 1, 1, 6400)), (1.0, (100, 8000), (1, 3, 1, 1, 8192))])
 def test_num_spikes_loss_fused_kernel_equals_the_tensor_expressions(Ts, region, shape):
     """The one-kernel numSpikes (value and gradient) against the tensor-expression form of the
     same module, which follows src/spikeLoss.py:85-104 line by line: loss within 1e-6, gradient
