@@ -6,19 +6,17 @@
 // reduction, writing two full-size temporaries; here g and out are read once (8 algorithmic
 // bytes per element, bound by HBM) and nothing but the [nNeurons] result is written.
 //
-// One CTA per neuron.  Its samples (all rows of the batch) are one sequence of chunks of V samples
-// dealt to the threads in turn, so that no lane idles at a row's end whatever T is; a thread asks for
-// kDelayGradAhead chunks of both arrays before it uses the first.  What bounds the pass is how many
-// requests are in flight: a layer has a few hundred neurons, two CTAs per SM at most.  The sample in
-// front of a chunk is the neighbouring lane's last one.  Partial sums are combined by warp shuffles
-// and a fixed-order pass over the warps' sums, so the result does not depend on scheduling.
-// (256 neurons, 32 x 2000 samples each: 51.7 -> 21.4 us; 512 neurons, 64 x 300: 20.1 -> 16.0 us, with one
-// CTA of eight warps per neuron and a row per warp before.)
+// One CTA of 1, 4, 8 or 16 warps per neuron.  Its samples (all rows of the batch) are one sequence of
+// chunks of V samples dealt to the threads in turn, so that no lane idles at a row's end whatever T is; a
+// thread asks for kDelayGradAhead chunks of both arrays before it uses the first.  What bounds the pass
+// is how many requests are in flight: a CTA large enough that a layer of a few hundred neurons fills
+// the chip, but no larger than the neuron's chunks and the other neurons leave work for (delay_grad_warps).
+// The sample in front of a chunk is the neighbouring lane's last one.  Partial sums are combined by warp
+// shuffles and a fixed-order pass over the warps' sums, so the result does not depend on scheduling.
 #include "common.cuh"
 
 namespace sb200 {
 
-constexpr int kDelayGradWarps = 16;
 constexpr int kDelayGradAhead = 4;
 
 template <int V>
@@ -33,13 +31,13 @@ __device__ __forceinline__ void load_chunk(float (&v)[V], const float *p)
 }
 
 // V = 4: rows on 16-byte boundaries (T % 4 == 0 and aligned arrays); V = 1: any
-template <int V>
-__global__ void __launch_bounds__(kDelayGradWarps * 32, 2)
+template <int V, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 32 / WARPS)
 delay_grad_kernel(float *__restrict__ grad_delay, const float *__restrict__ g, const float *__restrict__ out,
                   int64_t nBatch, int64_t nNeurons, int T, float Ts)
 {
-    constexpr int kThreads = kDelayGradWarps * 32;
-    __shared__ float warp_sum[kDelayGradWarps];
+    constexpr int kThreads = WARPS * 32;
+    __shared__ float warp_sum[WARPS];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const float f0 = -1.0f / Ts, f1 = 1.0f / Ts;
@@ -47,11 +45,13 @@ delay_grad_kernel(float *__restrict__ grad_delay, const float *__restrict__ g, c
     const int64_t chunks = nBatch * per_row;
     const unsigned step_b = per_row ? kThreads / per_row : 0;    // kThreads chunks further on: rows and chunks
     const unsigned step_q = per_row ? kThreads % per_row : 0;
+    const unsigned b0 = per_row ? threadIdx.x / per_row : 0;     // this thread's first chunk of a neuron
+    const unsigned q0 = per_row ? threadIdx.x % per_row : 0;
 
     for (int64_t n = blockIdx.x; n < nNeurons; n += gridDim.x) {
         float acc[kDelayGradAhead] = {};
-        int64_t b = per_row ? threadIdx.x / per_row : 0;
-        unsigned q = per_row ? threadIdx.x % per_row : 0;
+        int64_t b = b0;
+        unsigned q = q0;
         for (int64_t c = warp * 32; c < chunks; c += kThreads * kDelayGradAhead) {      // uniform over the warp
             float gv[kDelayGradAhead][V], ov[kDelayGradAhead][V], before[kDelayGradAhead];
             bool ok[kDelayGradAhead], first[kDelayGradAhead];
@@ -91,16 +91,49 @@ delay_grad_kernel(float *__restrict__ grad_delay, const float *__restrict__ g, c
         for (int k = 0; k < kDelayGradAhead; ++k) sum += acc[k];
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-        if (lane == 0) warp_sum[warp] = sum;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            float total = 0.0f;
+        if constexpr (WARPS == 1) {
+            if (lane == 0) grad_delay[n] = sum * Ts;
+        } else {
+            if (lane == 0) warp_sum[warp] = sum;
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                float total = 0.0f;
 #pragma unroll
-            for (int w = 0; w < kDelayGradWarps; ++w) total += warp_sum[w];
-            grad_delay[n] = total * Ts;
+                for (int w = 0; w < WARPS; ++w) total += warp_sum[w];
+                grad_delay[n] = total * Ts;
+            }
+            __syncthreads();
         }
-        __syncthreads();
     }
+}
+
+// Warps per neuron (one warp: no barrier, 32 neurons at a time on an SM).  chunks: of one neuron.
+// Times in us with 1 / 4 / 8 / 16 warps (neurons: samples of each):
+//   16384: 1 x 300       14 /  27 /  43 /  80       one pass of a warp
+//   4096: 8 x 300        23 /  27 /  27 /  39       enough neurons, few passes
+//   512: 4 x 300         10 /   8 /   8 /  10       one pass of four warps
+//   8192: 8 x 1450      211 / 186 / 201 / 219       enough neurons, many passes
+//   512: 64 x 300        49 /  25 /  23 /  25       a few neurons per SM, a few passes
+//   512: 512 x 300      305 / 121 / 123 / 113       (5.6 TB/s)
+//   256: 32 x 2000      131 /  51 /  37 /  33       fewer than two neurons per SM
+static int delay_grad_warps(int64_t nNeurons, int64_t chunks)
+{
+    const int64_t sms = sm_count();
+    if (chunks <= 128 || (nNeurons >= 16 * sms && chunks <= 2048)) return 1;
+    if (chunks <= 1024 || nNeurons >= 8 * sms) return 4;
+    if (chunks <= 8192 && nNeurons >= 2 * sms) return 8;
+    return 16;
+}
+
+template <int V>
+static void launch_delay_grad(float *grad_delay, const float *g, const float *out, int64_t nBatch, int64_t nNeurons,
+                              int T, float Ts, cudaStream_t stream)
+{
+    const int warps = delay_grad_warps(nNeurons, nBatch * (T / V));
+    auto kern = warps == 1 ? delay_grad_kernel<V, 1> : warps == 4 ? delay_grad_kernel<V, 4>
+              : warps == 8 ? delay_grad_kernel<V, 8> : delay_grad_kernel<V, 16>;
+    const int64_t cap = (int64_t)sm_count() * 32;
+    kern<<<(unsigned)(nNeurons < cap ? nNeurons : cap), warps * 32, 0, stream>>>(grad_delay, g, out, nBatch, nNeurons, T, Ts);
 }
 
 }  // namespace sb200
@@ -115,15 +148,8 @@ extern "C" int slayer_b200_delay_grad(float *grad_delay, const float *grad_outpu
     if (nNeurons == 0) return SLAYER_B200_OK;
     SB200_REQUIRE(grad_delay != nullptr, "delay_grad: null pointer");
     SB200_REQUIRE(nBatch == 0 || T == 0 || (grad_output && output), "delay_grad: null pointer");
-    int64_t grid = nNeurons;
-    const int64_t cap = (int64_t)sm_count() * 32;
-    if (grid > cap) grid = cap;
     const bool vec = (T % 4 == 0) && aligned16(grad_output) && aligned16(output);
-    if (vec)
-        delay_grad_kernel<4><<<(unsigned)grid, kDelayGradWarps * 32, 0, (cudaStream_t)stream>>>(
-            grad_delay, grad_output, output, nBatch, nNeurons, (int)T, Ts);
-    else
-        delay_grad_kernel<1><<<(unsigned)grid, kDelayGradWarps * 32, 0, (cudaStream_t)stream>>>(
-            grad_delay, grad_output, output, nBatch, nNeurons, (int)T, Ts);
+    (vec ? launch_delay_grad<4> : launch_delay_grad<1>)(grad_delay, grad_output, output, nBatch, nNeurons, (int)T, Ts,
+                                                        (cudaStream_t)stream);
     return check_launch("delay_grad kernel launch");
 }

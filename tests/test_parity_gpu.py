@@ -721,6 +721,21 @@ def test_delay_grad(shape, Ts):
     np.testing.assert_array_equal(got, again)
 
 
+@pytest.mark.parametrize("nb,nn,T", [(1, 5000, 512), (3, 4900, 7), (7, 2400, 1000),       # one warp per neuron
+                                     (1, 1000, 516), (3, 4800, 999),                       # four
+                                     (8, 300, 1000), (2, 1000, 1025),                      # eight
+                                     (33, 290, 1000), (5, 64, 2000), (1, 3, 1027)])        # sixteen
+def test_delay_grad_over_its_numbers_of_warps(nb, nn, T):
+    rng = np.random.RandomState(nn + T)
+    g = rng.randn(nb, nn, T).astype(np.float32)
+    out = (rng.randn(nb, nn, T) * (rng.rand(nb, nn, T) < 0.4)).astype(np.float32)
+    got = G.host(G.c_delay_grad(G.dev(g), G.dev(out), 1.0))
+    want = co.delay_grad(g, out, 1.0).ravel()
+    # a chain of at most 64 rounded sums, a tree of ten and two roundings of each term
+    terms = np.abs(g) * (np.abs(out) + np.abs(np.pad(out, ((0, 0), (0, 0), (1, 0)))[..., :-1]))
+    assert np.all(np.abs(got - want) <= 80 * 2.0 ** -24 * terms.sum((0, 2)))
+
+
 def test_delay_grad_unaligned_and_empty():
     rng = np.random.RandomState(5)
     g = rng.randn(3 * 4 * 300 + 1).astype(np.float32)
