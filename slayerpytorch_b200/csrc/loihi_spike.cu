@@ -196,8 +196,8 @@ __device__ __forceinline__ void wide_store_loihi(const float *tile_u, const floa
     const unsigned *mhalf = masks + (c16 >> 3) * kTile;
     const int c = (c16 & 7) * 4;
     const int64_t nrow = rows - row0;
+    int64_t at = (row0 + rsub) * (int64_t)T + (kWide * j + c16 * 4);
     if (wide_inner<SKEW>(row0, rows, j, T)) {
-        int64_t at = (row0 + rsub) * (int64_t)T + (kWide * j + c16 * 4);
 #pragma unroll
         for (int i = 0; i < kTile / 2; ++i, at += 2 * (int64_t)T) {
             const int r = i * 2 + rsub;
@@ -212,33 +212,27 @@ __device__ __forceinline__ void wide_store_loihi(const float *tile_u, const floa
         return;
     }
 #pragma unroll
-    for (int i = 0; i < kTile / 2; ++i) {
+    for (int i = 0; i < kTile / 2; ++i, at += 2 * (int64_t)T) {
         const int r = i * 2 + rsub;
-        if (r >= nrow) continue;
-        const int t = kWide * j - (SKEW ? row_skew(skew0, r, T) : 0) + c16 * 4;
-        if (t >= T || t + 4 <= 0) continue;
+        const int skew = SKEW ? row_skew(skew0, r, T) : 0;
+        const int t = kWide * j + c16 * 4 - skew;
         const int wd = hoff + tile_word(r, c);
-        const float4 vu = WRITE_U ? *reinterpret_cast<const float4 *>(tile_u + wd) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        const float4 vv = WRITE_V ? *reinterpret_cast<const float4 *>(tile_v + wd) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        const int64_t off = at - skew;
         const unsigned m = mhalf[r] >> c;
-        const float4 vs = make_float4((m & 1u) ? 1.0f : 0.0f, (m & 2u) ? 1.0f : 0.0f, (m & 4u) ? 1.0f : 0.0f, (m & 8u) ? 1.0f : 0.0f);
-        const int64_t off = (row0 + r) * (int64_t)T + t;
-        if (t >= 0 && t + 4 <= T) {
-            if (WRITE_U) *reinterpret_cast<float4 *>(gu + off) = vu;
-            if (WRITE_V) *reinterpret_cast<float4 *>(gv + off) = vv;
-            *reinterpret_cast<float4 *>(gs + off) = vs;
-        } else {
-            const float eu[4] = {vu.x, vu.y, vu.z, vu.w};
-            const float ev[4] = {vv.x, vv.y, vv.z, vv.w};
-            const float es[4] = {vs.x, vs.y, vs.z, vs.w};
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (t + k >= 0 && t + k < T) {
-                    if (WRITE_U) gu[off + k] = eu[k];
-                    if (WRITE_V) gv[off + k] = ev[k];
-                    gs[off + k] = es[k];
-                }
+        if (r < nrow && t >= 0 && t + 4 <= T) {
+            if (WRITE_U) *reinterpret_cast<float4 *>(gu + off) = *reinterpret_cast<const float4 *>(tile_u + wd);
+            if (WRITE_V) *reinterpret_cast<float4 *>(gv + off) = *reinterpret_cast<const float4 *>(tile_v + wd);
+            *reinterpret_cast<float4 *>(gs + off) =
+                make_float4((m & 1u) ? 1.0f : 0.0f, (m & 2u) ? 1.0f : 0.0f, (m & 4u) ? 1.0f : 0.0f, (m & 8u) ? 1.0f : 0.0f);
         }
+    }
+    if (lane < nrow) {
+        const int64_t row = (row0 + lane) * (int64_t)T;
+        wide_row_ends<SKEW>(j, T, SKEW ? row_skew(skew0, lane, T) : 0, [&](int col, int t) {
+            if (WRITE_U) gu[row + t] = tile_u[wide_word(lane, col)];
+            if (WRITE_V) gv[row + t] = tile_v[wide_word(lane, col)];
+            gs[row + t] = (masks[(col >> 5) * kTile + lane] >> (col & 31) & 1u) ? 1.0f : 0.0f;
+        });
     }
 }
 
@@ -261,7 +255,7 @@ __device__ __forceinline__ void wide_store_loihi(const float *tile_u, const floa
 // the separate shift pass (8 bytes per element) disappears.
 // ---------------------------------------------------------------------------------------
 template <bool SKEW, bool WRITE_U, bool WRITE_V>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 loihi_get_spikes_wide_kernel(float *s, float *v, float *u, const float *w,
                              int64_t rows, int T, unsigned weightScale, int theta,
                              unsigned iKeep, unsigned vKeep, int vDecayMark, unsigned refDelay, int depth, int delay)

@@ -302,8 +302,10 @@ srm_get_spikes_kernel(float *s, float *u, const float *__restrict__ nu,
 // start are padded with -inf, which can neither spike nor be changed by a refractory tap, so
 // the skewed lanes idle through them with their state untouched.
 // ---------------------------------------------------------------------------------------
+// Two CTAs of up to eight warps must fit an SM: left to itself the compiler keeps the offsets of all rows of a
+// fill in 222 registers, and then one CTA of six warps does.
 template <int NB, int W, bool SKEW>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 srm_get_spikes_wide_kernel(float *s, float *u, const float *__restrict__ nu,
                            int64_t rows, int nuEff, int T, float theta, float spikeVal, int depth)
 {

@@ -237,17 +237,47 @@ constexpr int kWideWords = 2 * kTileWords;
 // number of wide tiles that cover a row of T samples for every skew (0..7)
 __host__ __device__ inline int skew_wide_tiles(int T) { return (T + 7 + kWide - 1) / kWide; }
 
-// true (for the whole warp) if every sample of the wide tile exists: then its fill and its drain
-// are straight runs of 16-byte accesses.  A warp's fill and drain are in series with its walk, and
-// only 8 to 13 warps fit an SM, so their length counts: with the bounds tested per access, a branch
-// each, a warp's accesses went out one at a time.  (Loihi 131072 x 1450, spikes only 460 -> 381 us;
-// 1048576 x 1450 with the voltage 4.49 -> 4.08 ms; SRM 191664 x 301 237 -> 217 us.)
+// true (for the whole warp) if every sample of the wide tile exists
 template <bool SKEW>
 __device__ __forceinline__ bool wide_inner(int64_t row0, int64_t rows, int j, int T)
 {
     return row0 + kTile <= rows && kWide * j >= (SKEW ? 7 : 0) && kWide * j + kWide <= T;
 }
 
+__device__ __forceinline__ int wide_word(int r, int c) { return (c >> 5) * kTileWords + tile_word(r, c & 31); }
+
+// The fills and drains below move the 16-byte chunks that lie wholly inside their rows, each under one
+// predicate (none where the whole tile exists); the samples of a row that share a chunk with its start or its
+// end are moved by the lane of that row, all rows at once.  A warp's fill and drain are in series with its walk, and at most
+// 12 warps fit an SM, so their length counts: with the kinds of chunk told apart at every access, each
+// access was a branch of its own.  (us, so / now: Loihi delayed 262144 x 33 84 / 59, 65536 x 301 92 / 74,
+// 131072 x 1450 648 / 570; SRM 65536 x 50 41 / 23, 191664 x 301 244 / 176, 8192 x 1999 240 / 76.)
+//
+// f(column, time) for the samples of a row of this skew that share a chunk with samples outside the row: at most three
+// behind its start and three before its end
+template <bool SKEW, class F>
+__device__ __forceinline__ void wide_row_ends(int j, int T, int skew, F f)
+{
+    const int past = T + skew - kWide * j;                // column of the first sample after the row
+    if (SKEW && j == 0 && (skew & 3)) {
+#pragma unroll
+        for (int e = 1; e < 4; ++e) {
+            const int c = (skew & ~3) + e;
+            if (c >= skew && c < past) f(c, c - skew);
+        }
+    }
+    if (past > 0 && past < kWide) {
+        const int first = SKEW && j == 0 ? (skew + 3) & ~3 : 0;      // what lies before is dealt with above
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+            const int c = (past & ~3) + e;
+            if (c >= first && c < past) f(c, kWide * j + c - skew);
+        }
+    }
+}
+
+// Samples in front of a row's start are filled with `pad`.  What stands behind a row's end in a chunk that the
+// row's last samples share is not written (and never used: the walk's results there are not stored).
 template <bool SKEW = true>
 __device__ __forceinline__ void wide_prefetch_skew(float *tile, const float *g, int64_t row0, int64_t rows,
                                                    int j, int T, int lane, int skew0, float pad)
@@ -257,8 +287,8 @@ __device__ __forceinline__ void wide_prefetch_skew(float *tile, const float *g, 
     float *half = tile + (c16 >> 3) * kTileWords;
     const int c = (c16 & 7) * 4;                // column inside the half
     const int64_t nrow = rows - row0;
+    const float *src = g + (row0 + rsub) * (int64_t)T + (kWide * j + c16 * 4);
     if (wide_inner<SKEW>(row0, rows, j, T)) {
-        const float *src = g + (row0 + rsub) * (int64_t)T + (kWide * j + c16 * 4);
 #pragma unroll
         for (int i = 0; i < kTile / 2; ++i, src += 2 * (int64_t)T) {
             const int r = i * 2 + rsub;
@@ -267,38 +297,22 @@ __device__ __forceinline__ void wide_prefetch_skew(float *tile, const float *g, 
         return;
     }
 #pragma unroll
-    for (int i = 0; i < kTile / 2; ++i) {
+    for (int i = 0; i < kTile / 2; ++i, src += 2 * (int64_t)T) {
         const int r = i * 2 + rsub;
-        const int t = kWide * j - (SKEW ? row_skew(skew0, r, T) : 0) + c16 * 4;      // time of the chunk's first sample
-        float *dst = half + tile_word(r, c);
-        const float *src = g + (row0 + r) * (int64_t)T + t;
-        if (r >= nrow || t >= T) {
-            cp_async<16>(dst, g, false);
-        } else if (t >= 0 && t + 4 <= T) {
-            cp_async<16>(dst, src, true);
-        } else if (t + 4 <= 0) {
-            *reinterpret_cast<float4 *>(dst) = make_float4(pad, pad, pad, pad);
-        } else {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                if (t + e < 0) dst[e] = pad;
-                else cp_async<4>(dst + e, (t + e < T) ? src + e : g, t + e < T);
-            }
-        }
+        const int skew = SKEW ? row_skew(skew0, r, T) : 0;
+        const int t = kWide * j + c16 * 4 - skew;          // time of the chunk's first sample
+        const bool whole = r < nrow && t >= 0 && t + 4 <= T;
+        if (whole || r >= nrow || t >= T) cp_async<16>(half + tile_word(r, c), whole ? src - skew : g, whole);
     }
-}
-
-// Store four samples starting at time t of a row (clipped to [0, T)).
-__device__ __forceinline__ void store_clipped4(float *row, int t, int T, const float4 &v)
-{
-    if (t >= T || t + 4 <= 0) return;
-    if (t >= 0 && t + 4 <= T) {
-        *reinterpret_cast<float4 *>(row + t) = v;
-    } else {
-        const float e[4] = {v.x, v.y, v.z, v.w};
+    if (lane < nrow) {
+        const int skew = SKEW ? row_skew(skew0, lane, T) : 0;
+        const float *row = g + (row0 + lane) * (int64_t)T;
+        if (SKEW && j == 0) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (t + k >= 0 && t + k < T) row[t + k] = e[k];
+            for (int e = 0; e < 7; ++e)
+                if (e < skew) tile[tile_word(lane, e)] = pad;
+        }
+        wide_row_ends<SKEW>(j, T, skew, [&](int col, int t) { cp_async<4>(tile + wide_word(lane, col), row + t, true); });
     }
 }
 
@@ -312,8 +326,8 @@ __device__ __forceinline__ void wide_store_skew(const float *tile, float *g, int
     const float *half = tile + (c16 >> 3) * kTileWords;
     const int c = (c16 & 7) * 4;
     const int64_t nrow = rows - row0;
+    float *dst = g + (row0 + rsub) * (int64_t)T + (kWide * j + c16 * 4);
     if (wide_inner<SKEW>(row0, rows, j, T)) {
-        float *dst = g + (row0 + rsub) * (int64_t)T + (kWide * j + c16 * 4);
 #pragma unroll
         for (int i = 0; i < kTile / 2; ++i, dst += 2 * (int64_t)T) {
             const int r = i * 2 + rsub;
@@ -323,11 +337,17 @@ __device__ __forceinline__ void wide_store_skew(const float *tile, float *g, int
         return;
     }
 #pragma unroll
-    for (int i = 0; i < kTile / 2; ++i) {
+    for (int i = 0; i < kTile / 2; ++i, dst += 2 * (int64_t)T) {
         const int r = i * 2 + rsub;
-        if (r >= nrow || !(changed >> r & 1u)) continue;
-        const int t = kWide * j - (SKEW ? row_skew(skew0, r, T) : 0) + c16 * 4;
-        store_clipped4(g + (row0 + r) * (int64_t)T, t, T, *reinterpret_cast<const float4 *>(half + tile_word(r, c)));
+        const int skew = SKEW ? row_skew(skew0, r, T) : 0;
+        const int t = kWide * j + c16 * 4 - skew;
+        const float4 v = *reinterpret_cast<const float4 *>(half + tile_word(r, c));
+        if (r < nrow && t >= 0 && t + 4 <= T && (changed >> r & 1u)) *reinterpret_cast<float4 *>(dst - skew) = v;
+    }
+    if (lane < nrow && (changed >> lane & 1u)) {
+        float *row = g + (row0 + lane) * (int64_t)T;
+        wide_row_ends<SKEW>(j, T, SKEW ? row_skew(skew0, lane, T) : 0,
+                            [&](int col, int t) { row[t] = tile[wide_word(lane, col)]; });
     }
 }
 
@@ -342,8 +362,8 @@ __device__ __forceinline__ void wide_store_spikes_skew(const unsigned *masks, fl
     const unsigned *half = masks + (c16 >> 3) * kTile;
     const int sh = (c16 & 7) * 4;
     const int64_t nrow = rows - row0;
+    float *dst = g + (row0 + rsub) * (int64_t)T + (kWide * j + c16 * 4);
     if (wide_inner<SKEW>(row0, rows, j, T)) {
-        float *dst = g + (row0 + rsub) * (int64_t)T + (kWide * j + c16 * 4);
 #pragma unroll
         for (int i = 0; i < kTile / 2; ++i, dst += 2 * (int64_t)T) {
             const int r = i * 2 + rsub;
@@ -354,14 +374,20 @@ __device__ __forceinline__ void wide_store_spikes_skew(const unsigned *masks, fl
         return;
     }
 #pragma unroll
-    for (int i = 0; i < kTile / 2; ++i) {
+    for (int i = 0; i < kTile / 2; ++i, dst += 2 * (int64_t)T) {
         const int r = i * 2 + rsub;
-        if (r >= nrow) continue;
-        const int t = kWide * j - (SKEW ? row_skew(skew0, r, T) : 0) + c16 * 4;
+        const int skew = SKEW ? row_skew(skew0, r, T) : 0;
+        const int t = kWide * j + c16 * 4 - skew;
         const unsigned m = half[r] >> sh;
-        store_clipped4(g + (row0 + r) * (int64_t)T, t, T,
-                       make_float4((m & 1u) ? value : 0.0f, (m & 2u) ? value : 0.0f,
-                                   (m & 4u) ? value : 0.0f, (m & 8u) ? value : 0.0f));
+        if (r < nrow && t >= 0 && t + 4 <= T)
+            *reinterpret_cast<float4 *>(dst - skew) =
+                make_float4((m & 1u) ? value : 0.0f, (m & 2u) ? value : 0.0f, (m & 4u) ? value : 0.0f, (m & 8u) ? value : 0.0f);
+    }
+    if (lane < nrow) {
+        float *row = g + (row0 + lane) * (int64_t)T;
+        wide_row_ends<SKEW>(j, T, SKEW ? row_skew(skew0, lane, T) : 0, [&](int col, int t) {
+            row[t] = (masks[(col >> 5) * kTile + lane] >> (col & 31) & 1u) ? value : 0.0f;
+        });
     }
 }
 

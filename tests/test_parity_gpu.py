@@ -10,6 +10,7 @@ import pytest
 import torch
 
 from oracle import cpu_oracle as co
+from slayerpytorch_b200 import capi
 from tests import gpu_util as G
 
 pytestmark = pytest.mark.gpu
@@ -478,6 +479,49 @@ def test_loihi_get_spikes_delayed_equals_get_spikes_then_shift(T, delay):
     np.testing.assert_array_equal(G.host(d), G.host(G.c_shift_scalar(s, delay, 1.0)))
     np.testing.assert_array_equal(G.host(G.c_loihi_spikes_only(wd, *params, delay)), want_d)
     assert T < 30 or s_o.sum() > 0
+
+
+@pytest.mark.parametrize("T", [1, 2, 3, 5, 6, 7, 9, 12, 31, 58, 61, 63, 65, 66, 71, 121, 127, 129, 135])
+def test_row_skewed_tiles_write_their_rows_and_nothing_else(T):
+    """Rows that start and end inside 16-byte chunks, from arrays on 16- and 32-byte boundaries, in memory that must
+    stay as it is in front of and behind them; the last row block has five rows."""
+    rng = np.random.RandomState(T)
+    rows, pad = 37, 16
+    u = (rng.randn(rows, T) * 8).astype(np.float32)
+    nu = np.array([0.0, -20.0, -14.7, -8.1, -3.98, -1.83], np.float32)
+    w = (np.round((rng.rand(rows, T) - 0.5) * 200) * (rng.rand(rows, T) < 0.4)).astype(np.float32)
+    params = (0, 5120, 1024, 128, 2)
+    s_o, u_o = co.srm_get_spikes(u, nu, 10.0, 1.0)
+    loihi_o = co.loihi_get_spikes(w, *params)
+    delayed_o = co.shift(loihi_o[0], 1.0, 1.0)
+    for off in (4, 8):
+        def framed(values=None):
+            memory = torch.full((pad + off + rows * T + pad,), 77.0, device="cuda")
+            view = memory[pad + off:pad + off + rows * T]
+            if values is not None:
+                view.copy_(torch.from_numpy(values).reshape(-1))
+            return memory, view
+
+        def check(frame, want):
+            memory, view = frame
+            assert_same_floats(G.host(view).reshape(rows, T), want)
+            outside = torch.cat((memory[:pad + off], memory[pad + off + rows * T:]))
+            assert bool((outside == 77.0).all())
+
+        fu, fs, fw = framed(u), framed(), framed(w)
+        capi.call("slayer_b200_srm_get_spikes", G.ptr(fs[1]), G.ptr(fu[1]), G.ptr(G.dev(nu)), rows, nu.size, T, 10.0, 1.0, G.stream())
+        check(fs, s_o)
+        check(fu, u_o)
+        outs = [framed() for _ in range(3)]
+        capi.call("slayer_b200_loihi_get_spikes", *[G.ptr(o[1]) for o in outs], G.ptr(fw[1]), rows, T, *params, G.stream())
+        for frame, want in zip(outs, loihi_o):
+            check(frame, want)
+        d, v, only = framed(), framed(), framed()
+        capi.call("slayer_b200_loihi_get_spikes_delayed", G.ptr(d[1]), G.ptr(v[1]), None, G.ptr(fw[1]), rows, T, *params, 1, G.stream())
+        capi.call("slayer_b200_loihi_spikes_only", G.ptr(only[1]), G.ptr(fw[1]), rows, T, *params, 1, G.stream())
+        check(d, delayed_o)
+        check(v, loihi_o[1])
+        check(only, delayed_o)
 
 
 @pytest.mark.parametrize("off,T,delay,theta", [(0, 65, 0, 5120), (0, 65, 64, 5120), (1, 63, 0, 5120), (1, 129, 2, 5120),
