@@ -315,7 +315,14 @@ def test_num_spikes_loss_against_a_host_restatement():
 
 @pytest.mark.parametrize("Ts,region,shape", [(1.0, (0, 300), (64, 10, 1, 1, 300)), (1.0, (40, 260), (5, 10, 1, 1, 300)),
                                              (0.5, (10, 120), (3, 4, 2, 2, 300)), (1.0, (0, 2000), (2, 7, 1, 1, 2000)),
-                                             (1.0, (0, 6400), (2, 3, 1, 1, 6400)), (1.0, (100, 8000), (1, 3, 1, 1, 8192))])
+                                             (1.0, (0, 6400), (2, 3, 1, 1, 6400)), (1.0, (100, 8000), (1, 3, 1, 1, 8192)),
+                                             # one row or several for a CTA of one warp or of four
+                                             (1.0, (0, 2), (512, 10, 1, 1, 2)), (1.0, (3, 90), (500, 10, 1, 1, 96)),
+                                             (1.0, (70, 257), (600, 10, 1, 1, 256)), (1.0, (0, 200), (512, 5, 1, 1, 257)),
+                                             # the ends of groups of 32 steps and of a warp's 128
+                                             (1.0, (0, 20), (3, 4, 1, 1, 31)), (1.0, (5, 60), (3, 4, 1, 1, 65)),
+                                             (1.0, (0, 127), (3, 4, 1, 1, 127)), (1.0, (100, 128), (3, 4, 1, 1, 128)),
+                                             (1.0, (0, 64), (3, 4, 1, 1, 129)), (1.0, (200, 513), (3, 4, 1, 1, 513))])
 def test_num_spikes_loss_fused_kernel_equals_the_tensor_expressions(Ts, region, shape):
     """The one-kernel numSpikes (value and gradient) against the tensor-expression form of the
     same module, which follows src/spikeLoss.py:85-104 line by line: loss within 1e-6, gradient
@@ -343,6 +350,17 @@ def test_num_spikes_loss_fused_kernel_equals_the_tensor_expressions(Ts, region, 
     torch.testing.assert_close(la, lb, rtol=1e-6, atol=0)
     torch.testing.assert_close(ga, gb, rtol=1e-5, atol=1e-5 * gb.abs().max().item())
     assert ga.abs().sum() > 0
+
+
+def test_num_spikes_loss_operator_uses_no_taps_beyond_the_row():
+    sc, _ = slayerpytorch_b200.load_ops()
+    g = torch.Generator(device="cuda").manual_seed(4)
+    for shape in ((3, 4, 40), (1000, 5, 40)):
+        s = (torch.rand(shape, device="cuda", generator=g) < 0.2).float()
+        desired = torch.randint(0, 9, (shape[0] * shape[1],), device="cuda", generator=g).float()
+        taps = torch.rand(90, device="cuda", generator=g)
+        long, cut = (sc.numSpikesLoss(s, desired, f, 10, 30, 1.0, 1.0) for f in (taps, taps[:40].contiguous()))
+        assert all(torch.equal(a, b) for a, b in zip(long, cut)) and long[0] > 0
 
 
 def test_loihi_spike_delayed_layer_function_equals_the_two_steps():
