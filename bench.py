@@ -107,7 +107,7 @@ def measured_peak_gbs():
 
 # ------------------------------------------------------------------------ response kernels
 def srm_kernels(T, Ts=1.0, tauSr=None):
-    from slayerpytorch_b200.layer import alpha_kernel
+    from slayerpytorch_b200.response import alpha_kernel
     n = SRM_NEURON
     srm = torch.tensor(alpha_kernel(tauSr or n["tauSr"], Ts, T * Ts), dtype=torch.float32)
     ref = torch.tensor(alpha_kernel(n["tauRef"], Ts, T * Ts, mult=-n["scaleRef"] * n["theta"]), dtype=torch.float32)
@@ -115,7 +115,7 @@ def srm_kernels(T, Ts=1.0, tauSr=None):
 
 
 def loihi_kernel():
-    from slayerpytorch_b200.layer import loihi_psp_kernel
+    from slayerpytorch_b200.response import loihi_psp_kernel
     return torch.tensor(loihi_psp_kernel(LOIHI_NEURON), dtype=torch.float32)
 
 

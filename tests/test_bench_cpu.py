@@ -2,6 +2,7 @@
 bound and which convs the probe would send to the event-driven kernel - on small workloads built
 with the oracle as the operator set (no GPU, no CUDA extension)."""
 import os
+import subprocess
 import sys
 
 import pytest
@@ -56,3 +57,17 @@ def test_probe_rule_and_bound_of_an_event_driven_conv():
     assert set(bench.SPARSE_DENSITY) == {"conv", "convPacked"}
     for op in bench.ALG_BYTES:
         assert bench.kernel_of(op, 300) and bench.kernel_of(op, 1450)
+
+
+def test_the_reference_arm_maps_none_of_this_packages_libraries():
+    script = """
+import argparse
+import bench
+args = argparse.Namespace(config=1, steps=1, warmup=0, no_reference_cuda=True, scaling="strong")
+assert bench.time_reference(args, 0, 1)["value"] > 0
+maps = open("/proc/self/maps").read()
+assert "libslayer_oracle" in maps
+assert "slayer_b200.so" not in maps and "slayerCuda" not in maps and "slayerLoihiCuda" not in maps
+"""
+    done = subprocess.run([sys.executable, "-c", script], cwd=ROOT, capture_output=True, text=True)
+    assert done.returncode == 0, done.stderr
