@@ -209,3 +209,30 @@ def test_loihi_first_layer_shape_rows_match_oracle():
     finally:
         co.set_ftz(False)
         torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("T", [130, 184])                # rows on and off 32-byte boundaries
+def test_loihi_forms_with_fewer_outputs_over_several_row_blocks_per_warp(T):
+    """Enough rows that every warp walks several row blocks with the shallow prefetch: the forms without the current
+    and without the voltage against getSpikes and shift (all elements), and those against the oracle (a sample)."""
+    sc, lc = slayerpytorch_b200.load_ops()
+    dev = torch.device("cuda")
+    rows = 131072 + 5
+    g = torch.Generator(device=dev).manual_seed(T)
+    w = torch.randint(-128, 128, (rows, T), device=dev, generator=g).float()
+    w.mul_(torch.rand(rows, T, device=dev, generator=g) < 0.2)
+    params = (0, 5120, 1024, 128, 2)
+    s, v, _ = lc.getSpikes(w, *params)
+    idx_np = np.unique(np.concatenate(([0, 31, 32, rows - 6, rows - 1], np.random.RandomState(1).randint(0, rows, 300))))
+    idx = torch.from_numpy(idx_np).to(dev)
+    s_o, v_o, _ = co.loihi_get_spikes(w[idx].cpu().numpy(), *params)
+    np.testing.assert_array_equal(s[idx].cpu().numpy(), s_o)
+    np.testing.assert_array_equal(v[idx].cpu().numpy(), v_o)
+    assert s_o.mean() > 0.001
+    for delay in (0, 1, 63):
+        want = sc.shift(s, float(delay), 1.0)
+        (only,) = lc.getSpikesDelayed(w, *params, delay, False, False)
+        assert torch.equal(only, want)
+        del only
+        delayed, voltage = lc.getSpikesDelayed(w, *params, delay)
+        assert torch.equal(delayed, want) and torch.equal(voltage, v)
