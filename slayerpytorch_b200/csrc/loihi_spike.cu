@@ -149,7 +149,7 @@ loihi_get_spikes_kernel(float *s, float *v, float *u, const float *w,
 
 
 // One time step of the neuron for one row.  The decays are written on the magnitude with the
-// sign folded back in by xor / subtract (sm = 0 or -1): for every 32-bit state, INT_MIN
+// sign (us, vs = 0 or all ones) folded back in by xor and subtract: for every 32-bit state, INT_MIN
 // included, this is the reference's expression sgn(x) * ((sgn(x) * x * keep) >> 12) evaluated
 // modulo 2^32 with a logical shift.  A row's steps are a serial chain, and a scheduler has two or
 // three rows' chains to interleave, so what need not be on it is not: the magnitude is a maximum,
@@ -247,9 +247,9 @@ __device__ __forceinline__ void wide_store_loihi(const float *tile_u, const floa
 // what the definition prescribes for t = 0 (0 > theta cannot fire because theta >= 0 here).
 //
 // WRITE_U = false leaves the current out (callers that only keep spikes and voltage: 12 instead
-// of 16 bytes per element), WRITE_V = false the voltage too (no gradient: 8 bytes, and without the
-// voltage tile 13 warps instead of 8 per SM).  131072 x 1450, spikes then shift, no gradient:
-// 1143 -> 781 us.  `delay` (0 .. 63 steps) writes the spikes already delayed,
+// of 16 bytes per element), WRITE_V = false the voltage too (an input that requires no gradient: 8 bytes,
+// and without the voltage tile 12 warps instead of 8 per SM).  131072 x 1450 (events): 769 us with three
+// outputs, 568 (4.0 TB/s) with two, 368 (4.1 TB/s) with the spikes alone.  `delay` (0 .. 63 steps) writes the spikes already delayed,
 // s_out[t] = s[t - delay]: a Loihi layer is always followed by a delay of one step, and the
 // spike bits of a tile only need a 64-bit shift with carry from the previous tile for that, so
 // the separate shift pass (8 bytes per element) disappears.

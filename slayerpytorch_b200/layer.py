@@ -199,7 +199,8 @@ class _LoihiSpikeFunction(torch.autograd.Function):
     @staticmethod
     def delayed(ctx, weightedSpikes, neuron, Ts, steps):
         """The spikes, ``steps`` late, and what the backward needs of the neuron: the voltage, or nothing
-        where no gradient flows (12 or 8 bytes per element instead of 16)."""
+        if the input requires no gradient (12 or 8 bytes per element instead of 16).  An input that requires
+        one keeps its voltage under ``torch.no_grad()`` too."""
         if weightedSpikes.dtype == torch.int32:
             Ts = 1
         w = weightedSpikes if Ts == 1 and weightedSpikes.dtype == torch.float32 else (weightedSpikes * Ts).float()
