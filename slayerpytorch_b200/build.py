@@ -9,6 +9,7 @@ Products, all under ``slayerpytorch_b200/lib/``:
 Run ``python -m slayerpytorch_b200.build`` (add ``-v`` for ptxas resource usage, ``-f`` to
 force a rebuild).
 """
+import concurrent.futures
 import os
 import subprocess
 import sys
@@ -75,16 +76,18 @@ def build_library(force=False, verbose=False):
     os.makedirs(LIBDIR, exist_ok=True)
     os.makedirs(OBJDIR, exist_ok=True)
     hdrs = [h if os.path.isabs(h) else os.path.join(CSRC, h) for h in HEADERS]
-    objs = []
-    relink = force
+    objs, compile_cmds = [], []
     for src, extra in CUDA_SOURCES.items():
         s = os.path.join(CSRC, src)
         o = os.path.join(OBJDIR, src.replace(".cu", ".o"))
         if force or _newer(o, [s] + hdrs + [os.path.abspath(__file__)]):
             flags = ["-Xptxas", "-v"] if verbose else []
-            _run([nvcc()] + ARCH + NVCC_COMMON + extra + flags + ["-c", s, "-o", o], verbose)
-            relink = True
+            compile_cmds.append([nvcc()] + ARCH + NVCC_COMMON + extra + flags + ["-c", s, "-o", o])
         objs.append(o)
+    # side by side: two of the sources take a few minutes each
+    with concurrent.futures.ThreadPoolExecutor(max_workers=os.cpu_count() or 1) as pool:
+        list(pool.map(lambda cmd: _run(cmd, verbose), compile_cmds))
+    relink = force or bool(compile_cmds)
     lib = os.path.join(LIBDIR, "libslayer_b200.so")
     if relink or not os.path.isfile(lib):
         _run([nvcc()] + ARCH + ["-shared", "-o", lib] + objs, verbose)
